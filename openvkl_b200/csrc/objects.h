@@ -19,6 +19,7 @@
 
 #include "../../include/openvkl_cuda.h"
 #include "grid.h"
+#include "kernels.h"
 
 namespace vklcuda {
 

@@ -215,32 +215,68 @@ bool binned(Device *d, Sampler *s, int filter, uint64_t n, const float *pts, uin
 // The layout of a large call's points, where it decides the kernel
 // (k_sample_rays.cu): detected once per call, on its first chunk.
 struct CallLayout : PointLayout {
-  bool known = false;
+  bool known         = false;
+  LayoutSlots *slots = nullptr;  // holder of `device`
+  int slot           = -1;
+  cudaStream_t stream = nullptr;
+  CallLayout()        = default;
+  CallLayout(const CallLayout &) = delete;
+  CallLayout &operator=(const CallLayout &) = delete;
+  ~CallLayout()
+  {
+    if (slot >= 0)
+      releaseLayout(*slots, slot, stream);
+  }
 };
 
+// Which calls look for it:
+//  - dense float, from 2^20 points: the call waits for the answer.  The
+//    detector's 12 us are half of the fastest such call (1.5M camera-ray
+//    samples 33 us with it, without detector and in sorted tiles 45 to 57);
+//  - temporally varying voxels larger than the 126 MB L2, from 12.6M points,
+//    without waiting (floats x 4 times, 14M samples: 205 MB of voxels, 64 per
+//    ray 288 -> 262 us, 200 per ray 377 -> 303; the detector costs points in
+//    no order 989 -> 1000, rays of 12 samples 141 -> 158.  Smaller voxels by
+//    rays are no faster than point by point: 27 MB 211 and 223).
+// No other call's kernel depends on it.  (Types other than float chosen on the
+// device, each kernel returning where another applies, from 17M points: 50M
+// camera-ray samples of shorts, 96 per ray, 448 us, in sorted tiles 417.)
 void findLayout(Device *d, Sampler *s, int filter, uint64_t n, const float *pts, uint32_t attr, CallLayout &layout)
 {
   const DevGrid &g = s->volume->grid;
-  // From where the detector's 12 us are a few per cent of the call: float
-  // attributes have the fastest run kernel, and the direct kernel suits the
-  // other types up to 2^22 points anyway.
-  const uint64_t least = g.temporal ? uint64_t(1) << 23 : g.type[attr] == VKL_FLOAT ? uint64_t(1) << 20 : uint64_t(1) << 22;
-  if (layout.known || !d->rayRuns || n < least || s->s.maxSamplingDepth < kNumLevels - 1 ||
-      !s->leafObservers.empty() || !layoutMatters(g, filter, s->s.maxSamplingDepth))
+  const bool waits = rayRunsApply(g, filter, attr) && n >= uint64_t(1) << 20;
+  const bool late  = g.temporal && filter == kFilterLinear && n >= uint64_t(3) << 22 &&
+                    s->volume->temporalBytes >= uint64_t(128) << 20;
+  if (!(waits || late) || layout.known || !d->rayRuns || s->s.maxSamplingDepth < kNumLevels - 1 ||
+      !s->leafObservers.empty())
     return;
   layout.known               = true;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaCheck(cudaStreamIsCapturing(d->stream, &cs), "capture status");
-  // the detector's answer is waited for: not while the stream is captured
+  // the detector's answer is waited for, or its slot: not while the stream is captured
   if (cs != cudaStreamCaptureStatusNone)
     return;
-  std::lock_guard<std::mutex> lock(d->runMutex);
-  (PointLayout &)layout = detectLayout(g, n, pts, d->runScratch, d->stream);
-  if (!rayRunsApply(g, filter, attr))
-    layout.S = 0;
-  if (layout.S > 0)
-    d->log(VKL_LOG_DEBUG, "sampling " + std::to_string(n) + " points as runs of " + std::to_string(layout.S) +
-                              " samples per ray\n");
+  PointLayout found;  // for the log
+  if (waits) {
+    std::lock_guard<std::mutex> lock(d->runMutex);
+    (PointLayout &)layout = found = detectLayout(g, n, pts, d->runScratch, d->stream);
+  } else {
+    layout.stream = d->stream;
+    layout.slots  = &d->layoutSlots;
+    layout.slot   = queueLayout(g, n, pts, d->layoutSlots, d->stream, layout);
+    if (layout.slot < 0 || d->logLevel > VKL_LOG_DEBUG)
+      return;
+    DeviceLayout l{};
+    cudaCheck(cudaMemcpyAsync(&l, layout.device, sizeof(l), cudaMemcpyDeviceToHost, d->stream), "layout log");
+    cudaCheck(cudaStreamSynchronize(d->stream), "layout log");
+    found.order     = l.order >= kTemporalRays ? (int)l.order : 0;
+    found.scattered = !found.order;
+  }
+  const std::string how = found.S           ? "as runs of " + std::to_string(found.S) + " samples per ray"
+                          : found.order     ? "by rays of " + std::to_string(found.order) + " samples"
+                          : found.scattered ? "point by point"
+                                            : "in sorted tiles";
+  d->log(VKL_LOG_DEBUG, "sampling " + std::to_string(n) + " points " + how + "\n");
 }
 
 // Temporally varying volumes: points, times and results staged through the

@@ -15,14 +15,20 @@ namespace {
 //  - tricubic through an atlas (14.4M camera-ray samples 1004 -> 912 us; by
 //    rays 1047); with bricked loads the sort wins (double: 2.10 against 3.04
 //    ms);
-//  - trilinear, dense: by rays where the points come by rays (14.8M samples in
-//    40 per ray 202 us sorted, 159 by rays; double 288 and 248), point by
-//    point where they come in no order (10M: 585 -> 547 us), else the sort
-//    (12M samples 173 us against 283 point by point);
+//  - trilinear, dense float: by rays where the points come by rays (14.8M
+//    samples in 40 per ray 202 us sorted, 159 by rays), point by point where
+//    they come in no order (10M: 585 -> 547 us), else the sort (12M samples
+//    173 us against 283 point by point).  Other types keep the sort, which
+//    with the atlas is the fastest form that needs no knowledge of the layout
+//    (shorts, 600^3: 17M random points 795 us, 734 direct; camera rays of 12
+//    to 96 samples 192 to 228, 159 to 240 by the best of the float kernels for
+//    calls that wait for a detector; double, 4.2M camera-ray samples 81 to 182,
+//    88 to 180);
 //  - trilinear, sparse with a leaf map: direct (59M camera-ray samples 878 ->
-//    781 us, by rays 803; 16M random points 990 -> 620 us), but points in no
-//    order in stencil-block leaves, which are bound by DRAM and 4 % faster in
-//    tiles (885 against 922 us; camera rays 1018 -> 619 us);
+//    781 us, by rays 803; 16M random points 990 -> 620 us; stencil blocks,
+//    17M points over a 768^3 domain: random 545 us in tiles, 342 direct, camera
+//    rays 242 direct; only points that all lie in active leaves are 4 % faster
+//    in tiles, 885 against 922 us);
 //  - sparse without a leaf map and sparse tricubic keep the tiles.
 constexpr uint64_t kDirectPoints = uint64_t(1) << 20;
 
@@ -35,8 +41,7 @@ bool useDirect(const DevGrid &g, int filter, uint32_t maxDepth, uint64_t n, uint
     return true;
   if (g.dense)
     return filter == kFilterCubic ? tilesUseAtlas(g, attr) : layout.order || layout.scattered;
-  return filter == kFilterLinear && leafMapApplies(g, maxDepth) &&
-         !(layout.scattered && g.compress >= kCompressFP16Blocks);
+  return filter == kFilterLinear && leafMapApplies(g, maxDepth);
 }
 
 void dispatch(const DevGrid &g, int filter, uint32_t maxDepth, uint64_t n, const float *pts,

@@ -22,17 +22,15 @@ namespace {
 constexpr int kTemporalBlock = kDirectBlock;
 constexpr float kInfF     = __builtin_huge_valf();
 
-// S: samples per ray, where the points come by rays (directPoint): a warp's 32
-// points x 16 time samples are then close together (14.8M camera-ray samples
-// of 256x250x200 voxels x 4 steps: 425 -> 345 us).
+// LAYOUT: whether the points come by rays is read from `layout` (directPoint): a
+// warp's 32 points x 16 time samples are then close together (14.8M camera-ray
+// samples, 64 per ray, of 256x250x200 floats x 4 steps: 437 -> 335 us, 14M at
+// 200 per ray 377 -> 303).  Rays of fewer samples have them too far apart to
+// gain (40 per ray: 1.00 to 1.05 of the time point by point).
 template <typename T, int FILTER, bool GRAD>
-__global__ void __launch_bounds__(kTemporalBlock)
-    kSampleTemporal(const __grid_constant__ DevGrid g, uint32_t S, uint64_t n, const float *__restrict__ pts,
-                    const float *__restrict__ times, uint32_t attr, float *__restrict__ out)
+__device__ __forceinline__ void sampleTemporal(const DevGrid &g, uint64_t i, const float *__restrict__ pts,
+                                               const float *__restrict__ times, uint32_t attr, float *__restrict__ out)
 {
-  uint64_t i;
-  if (!directPoint(S, n, i))
-    return;
   const f3 p = xfmPoint(g.objectToIndex, loadPoint(pts, i));
   const TemporalDenseField<T> F(g, attr, times ? __ldg(times + i) : 0.f);
   if constexpr (GRAD) {
@@ -47,6 +45,18 @@ __global__ void __launch_bounds__(kTemporalBlock)
   } else {
     out[i] = filterAt<TemporalDenseField<T>, FILTER>(F, g.constantCellData != 0, p);
   }
+}
+
+template <typename T, int FILTER, bool GRAD, bool LAYOUT>
+__global__ void __launch_bounds__(kTemporalBlock)
+    kSampleTemporal(const __grid_constant__ DevGrid g, const DeviceLayout *__restrict__ layout, uint64_t n,
+                    const float *__restrict__ pts, const float *__restrict__ times, uint32_t attr,
+                    float *__restrict__ out)
+{
+  const uint32_t S = LAYOUT && layout->order >= kTemporalRays ? layout->order : 0u;
+  uint64_t i;
+  if (directPoint(blockIdx.x, S, n, i))
+    sampleTemporal<T, FILTER, GRAD>(g, i, pts, times, attr, out);
 }
 
 __global__ void __launch_bounds__(kTemporalBlock)
@@ -132,25 +142,20 @@ __global__ void __launch_bounds__(kTemporalBlock)
 
 template <typename T>
 void sampleTyped(const DevGrid &g, int filter, uint64_t n, const float *pts, const float *times, uint32_t attr,
-                 float *out, bool grad, uint32_t S, cudaStream_t st)
+                 float *out, bool grad, const DeviceLayout *layout, cudaStream_t st)
 {
-  const unsigned blocks = directBlocks(S, n);
-  if (filter == kFilterNearest) {
-    if (grad)
-      kSampleTemporal<T, kFilterNearest, true><<<blocks, kTemporalBlock, 0, st>>>(g, S, n, pts, times, attr, out);
-    else
-      kSampleTemporal<T, kFilterNearest, false><<<blocks, kTemporalBlock, 0, st>>>(g, S, n, pts, times, attr, out);
-  } else if (filter == kFilterCubic) {
-    if (grad)
-      kSampleTemporal<T, kFilterCubic, true><<<blocks, kTemporalBlock, 0, st>>>(g, S, n, pts, times, attr, out);
-    else
-      kSampleTemporal<T, kFilterCubic, false><<<blocks, kTemporalBlock, 0, st>>>(g, S, n, pts, times, attr, out);
-  } else {
-    if (grad)
-      kSampleTemporal<T, kFilterLinear, true><<<blocks, kTemporalBlock, 0, st>>>(g, S, n, pts, times, attr, out);
-    else
-      kSampleTemporal<T, kFilterLinear, false><<<blocks, kTemporalBlock, 0, st>>>(g, S, n, pts, times, attr, out);
-  }
+  // by rays a last group of 8 may be part empty
+  const unsigned blocks = directBlocks(0, n) + (layout ? kMaxRun * 8 / kDirectBlock : 0);
+  const auto k = [&] {
+    if (filter == kFilterNearest)
+      return grad ? kSampleTemporal<T, kFilterNearest, true, false> : kSampleTemporal<T, kFilterNearest, false, false>;
+    if (filter == kFilterCubic)
+      return grad ? kSampleTemporal<T, kFilterCubic, true, false> : kSampleTemporal<T, kFilterCubic, false, false>;
+    if (layout)
+      return grad ? kSampleTemporal<T, kFilterLinear, true, true> : kSampleTemporal<T, kFilterLinear, false, true>;
+    return grad ? kSampleTemporal<T, kFilterLinear, true, false> : kSampleTemporal<T, kFilterLinear, false, false>;
+  }();
+  k<<<blocks, kTemporalBlock, 0, st>>>(g, layout, n, pts, times, attr, out);
 }
 
 }  // namespace
@@ -161,7 +166,6 @@ void launchSampleTemporal(const DevGrid &g, int filter, uint64_t n, const float 
 {
   if (!n)
     return;
-  const uint32_t S = (uint32_t)layout.order;
   if (M > 1) {
     AttrList al{};
     al.count = M;
@@ -173,22 +177,22 @@ void launchSampleTemporal(const DevGrid &g, int filter, uint64_t n, const float 
     const uint32_t attr = attrs[0];
     switch (g.type[attr]) {
     case kUChar:
-      sampleTyped<uint8_t>(g, filter, n, points, times, attr, out, grad, S, st);
+      sampleTyped<uint8_t>(g, filter, n, points, times, attr, out, grad, layout.device, st);
       break;
     case kShort:
-      sampleTyped<int16_t>(g, filter, n, points, times, attr, out, grad, S, st);
+      sampleTyped<int16_t>(g, filter, n, points, times, attr, out, grad, layout.device, st);
       break;
     case kUShort:
-      sampleTyped<uint16_t>(g, filter, n, points, times, attr, out, grad, S, st);
+      sampleTyped<uint16_t>(g, filter, n, points, times, attr, out, grad, layout.device, st);
       break;
     case kHalf:
-      sampleTyped<__half>(g, filter, n, points, times, attr, out, grad, S, st);
+      sampleTyped<__half>(g, filter, n, points, times, attr, out, grad, layout.device, st);
       break;
     case kDouble:
-      sampleTyped<double>(g, filter, n, points, times, attr, out, grad, S, st);
+      sampleTyped<double>(g, filter, n, points, times, attr, out, grad, layout.device, st);
       break;
     default:
-      sampleTyped<float>(g, filter, n, points, times, attr, out, grad, S, st);
+      sampleTyped<float>(g, filter, n, points, times, attr, out, grad, layout.device, st);
     }
   }
   cudaCheck(cudaGetLastError(), "temporal sample kernel launch");

@@ -10,11 +10,22 @@
 namespace vklcuda {
 
 // The layout of a large call's points (detectLayout, k_sample_rays.cu).
+struct DeviceLayout;
 struct PointLayout {
   int S          = 0;      // samples per ray, where the ray-run kernel pays (0: elsewhere)
   int order      = 0;      // samples per ray, where going by rays is any closer together (0: elsewhere)
   bool scattered = false;  // no order at all
+  // The answer in device memory, where the call does not wait for it: the
+  // kernel queued behind the detector reads it (nullptr: the members above).
+  const DeviceLayout *device = nullptr;
 };
+struct DeviceLayout {
+  uint32_t order;  // PointLayout's
+};
+// Run lengths detectLayout looks for are below this.
+constexpr uint32_t kMaxRun = 2048;
+// Rays of a temporally varying volume's points, from where the kernel goes by them.
+constexpr uint32_t kTemporalRays = 48;
 
 // Sampling / gradients over N object-space points (AoS float3).  `attrs`
 // lists M attribute indices (M <= kMaxAttributes, host array); output is

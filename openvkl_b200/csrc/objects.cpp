@@ -718,7 +718,8 @@ void Volume::commitDense()
     }
     for (uint32_t a = 0; a < NA; ++a) {
       keep.emplace_back(attrs[a]);
-      grid.data[a] = attrs[a]->dev;
+      temporalBytes = attrs[a]->numItems * attrs[a]->itemSize;
+      grid.data[a]  = attrs[a]->dev;
       grid.type[a] = attrs[a]->type;
       if (atlases[a])
         device->giveAtlas(std::move(atlases[a]));

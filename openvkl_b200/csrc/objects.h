@@ -175,15 +175,41 @@ struct RunScratch {
   RunScratch &operator=(const RunScratch &) = delete;
   ~RunScratch();
 };
+// Scratch of detections that no call waits for: the detector's counters and
+// its answer, which the sampling kernels queued behind it read, so a call
+// holds a slot until its kernels have run.  `ready` is recorded behind them
+// on the call's stream and waited for (on the device) by the slot's next
+// user, which takes the slot its stream used last where it can: streams wait
+// for one another only when all slots are held by others.
+struct LayoutSlots {
+  static constexpr int kSlots = 16;
+  struct Slot {
+    cudaEvent_t ready   = nullptr;
+    cudaStream_t stream = nullptr;
+    uint64_t used       = 0;  // 0: never
+    bool taken          = false;
+  };
+  std::mutex mutex;
+  Slot slots[kSlots];
+  DeviceBuffer words;
+  uint64_t uses = 0;
+  LayoutSlots() = default;
+  LayoutSlots(const LayoutSlots &) = delete;
+  LayoutSlots &operator=(const LayoutSlots &) = delete;
+  ~LayoutSlots();
+};
 // Ray-run sampling of dense volumes with the trilinear filter: rayRunsApply
 // says whether the path covers the call, launchSampleRays samples (grad:
-// gradients) as launchSample / launchGradient do.  layoutMatters: the layout
-// decides the kernel of a large call (with or without ray runs);
-// detectLayout finds it (in sparse volumes only whether there is no order) and
-// waits for the stream to reach its answer.
+// gradients) as launchSample / launchGradient do.  detectLayout finds the
+// layout of a call's points and waits for the stream to reach its answer;
+// queueLayout leaves it in device memory for the kernels of the call, takes
+// the slot it is kept in and returns its index (-1: all are held, nothing was
+// queued), and releaseLayout gives the slot back behind those kernels.
 bool rayRunsApply(const DevGrid &g, int filter, uint32_t attr);
-bool layoutMatters(const DevGrid &g, int filter, uint32_t maxDepth);
 PointLayout detectLayout(const DevGrid &g, uint64_t n, const float *pts, RunScratch &scratch, cudaStream_t stream);
+int queueLayout(const DevGrid &g, uint64_t n, const float *pts, LayoutSlots &slots, cudaStream_t stream,
+                PointLayout &layout);
+void releaseLayout(LayoutSlots &slots, int slot, cudaStream_t stream);
 void launchSampleRays(const DevGrid &g, uint64_t n, const float *pts, uint32_t attr, float *out, bool grad, int S,
                       RunScratch &scratch, cudaStream_t stream);
 
@@ -248,6 +274,7 @@ struct Device {
   // device parameter "rayRunSampling" 0 turns the path off
   std::mutex runMutex;
   RunScratch runScratch;
+  LayoutSlots layoutSlots;
   bool rayRuns = true;
   bool binning = true;
   // Texture atlases of dense attributes (DevGrid::atlasTex): on by
@@ -335,6 +362,7 @@ struct Volume : ManagedObject {
   int gradientFilter = VKL_FILTER_LINEAR;
   uint32_t maxSamplingDepth = kNumLevels - 1;
   uint64_t levelNodes[kNumLevels] = {0, 0, 0, 0};
+  uint64_t temporalBytes = 0;  // of an attribute's voxels at all times, where they vary
 
   const char *typeName() const override { return isDense ? "structuredRegular" : "vdb"; }
   void commit() override;

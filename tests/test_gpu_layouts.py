@@ -23,9 +23,18 @@ def _voxels(dtype, dims=DIMS):
 
 def _points(order, n, hi):
     """n points by rays of `order` samples (an image 125 rays wide, the last
-    ray cut), or in no order."""
+    ray cut), in no order, or close together in no order by rays: each 2048
+    consecutive ones anywhere in one box of a few hundred sort bins."""
+    import torch
     if order == "none":
         return uniform_points_torch(n, (-1, -1, -1), hi, seed=6)
+    if order == "boxes":
+        g = torch.Generator(device="cuda")
+        g.manual_seed(7)
+        size = torch.tensor([64.0, 64.0, 32.0], device="cuda")
+        boxes = n // 2048 + 1
+        at = torch.rand((boxes, 1, 3), generator=g, device="cuda") * (torch.tensor(hi, device="cuda") - size)
+        return (at + torch.rand((boxes, 2048, 3), generator=g, device="cuda") * size).reshape(-1, 3)[:n].contiguous()
     return orbit_camera_samples_torch(125, n // (125 * order) + 1, order, (0, 0, 0), hi, seed=5)[:n].contiguous()
 
 
@@ -57,6 +66,19 @@ def _check(vkl, vol, log, route, pts, step, times=None):
         parts = torch.cat([call(pts[c].contiguous(), times=t(c)) for c in cut])
         assert not any("sampling" in m for m in log), log
         np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(parts.cpu().numpy()))
+
+
+@pytest.mark.parametrize("texture", [1, 0])
+@pytest.mark.parametrize("order,route", [(37, "as runs of 37 samples"), (19, "by rays of 19 samples"),
+                                         (24, "by rays of 24 samples"), ("none", "point by point"),
+                                         ("boxes", "in sorted tiles")])
+def test_float(vkl, order, route, texture):
+    """Rays whose warps touch up to 12 blocks of 16x16x2 voxels, up to 20, and
+    points of either other kind."""
+    dev, log = _logged(vkl, textureSampling=texture)
+    vol = vkl.structured_regular(dev, _voxels(np.float32), background=[0.5])
+    pts = _points(order, (1 << 20) + 5, tuple(float(d - 1) for d in DIMS))
+    _check(vkl, vol, log, route, pts, 500009)
 
 
 @pytest.mark.parametrize("dtype,texture", [(t, 1) for t in TYPES] + [(np.uint8, 0), (np.int16, 0)])

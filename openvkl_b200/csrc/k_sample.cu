@@ -44,6 +44,20 @@ bool useDirect(const DevGrid &g, int filter, uint32_t maxDepth, uint64_t n, uint
   return filter == kFilterLinear && leafMapApplies(g, maxDepth);
 }
 
+// Which calls for several attributes take the sorted tiles: a tile has a CTA
+// work through 1024 points and their attributes one after another, so it needs
+// some hundred thousand points to fill the GPU (four float attributes,
+// trilinear: 8,192 points 9.2 us with a thread per point, 13.8 in tiles; 65,536
+// even; 262,144 camera-ray samples 28 and 19).  Where the tile gathers with
+// plain loads it takes longer still (tricubic, double, four attributes: 8,192
+// camera-ray samples 37 us and 162; 262,144 172 and 208; 524,288 373 and 310).
+bool useTilesM(const DevGrid &g, int filter, uint32_t maxDepth, uint64_t n, uint32_t M, const uint32_t *attrs)
+{
+  const bool loads = g.dense ? filter == kFilterCubic && !tilesUseAtlas(g, attrs[0])
+                             : filter == kFilterCubic || !leafMapApplies(g, maxDepth);
+  return sameField(g, M, attrs) && n >= (uint64_t(1) << (loads ? 19 : 18));
+}
+
 void dispatch(const DevGrid &g, int filter, uint32_t maxDepth, uint64_t n, const float *pts,
               uint32_t attr, float *out, bool grad, const PointLayout &layout, cudaStream_t st)
 {
@@ -80,7 +94,7 @@ void launchSample(const DevGrid &g, int filter, uint32_t maxDepth, uint64_t n,
     al.count = M;
     for (uint32_t m = 0; m < M; ++m)
       al.a[m] = attrs[m];
-    if (!sameField(g, M, attrs))
+    if (!useTilesM(g, filter, maxDepth, n, M, attrs))
       launchSampleMixed(g, filter, maxDepth, n, points, al, out, stream);
     else if (filter == kFilterNearest)
       dispatchFilterM<kFilterNearest>(g, maxDepth, n, points, al, out, stream);

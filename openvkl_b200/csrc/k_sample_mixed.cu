@@ -1,6 +1,6 @@
-// Sampling of several attributes that differ in type (vklComputeSampleMN,
-// VdbSampler.ispc:131-252): one point per thread through the run-time
-// dispatch on type and filter.
+// Sampling of several attributes that differ in type, or at few points
+// (useTilesM, k_sample.cu) (vklComputeSampleMN, VdbSampler.ispc:131-252): one
+// point per thread through the run-time dispatch on type and filter.
 #include "sample_kernels.cuh"
 
 namespace vklcuda {

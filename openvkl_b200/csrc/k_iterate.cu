@@ -3,6 +3,10 @@
 // that lives in the caller's buffer by one step (the batched forms are in
 // k_intervals.cu and k_hits.cu).  Also the batched hit kernel of any voxel
 // type and filter, which shares their out-of-line sampling dispatch.
+
+// The filters are inlined at many call sites: the fused form of the tricubic
+// sums would give every kernel here its registers.
+#define VKL_TRICUBIC_PLAIN 1
 #include "iterate.cuh"
 #include "kernels.h"
 #include "objects.h"
@@ -19,8 +23,14 @@ __device__ __forceinline__ f3 ld3(const float *p, uint64_t i)
 }
 
 // Any voxel type and filter: one ray per thread through the out-of-line
-// sampling dispatch.
-__global__ void __launch_bounds__(kBlock) kHitsAny(const __grid_constant__ DevGrid g, uint32_t attr, int filter,
+// sampling dispatch.  CTAS per SM: 1 lets the march keep its 242 registers (two
+// are resident), 3 has it spill 576 bytes.  Rays that two per SM take at once
+// run 1.1 to 1.5 times as long spilled (20,000 rays through 300x280x310 bytes,
+// 1 to 20 isovalues); more rays of a march with few isovalues gain from the
+// third (200,000 rays, 1 isovalue 8.8 -> 7.3 ms; with 8 even, tricubic 0.85
+// times as fast).
+template <int CTAS>
+__global__ void __launch_bounds__(kBlock, CTAS) kHitsAny(const __grid_constant__ DevGrid g, uint32_t attr, int filter,
                                                    uint32_t depth, DevValueRanges vr, uint32_t numValues,
                                                    const float *__restrict__ values, uint64_t n,
                                                    const float *__restrict__ orgs, const float *__restrict__ dirs,
@@ -96,7 +106,12 @@ void launchHitsAny(const DevGrid &g, uint32_t attr, int filter, uint32_t depth, 
                    const float *directions, const float *tRanges, uint32_t maxPerRay, DevHit *out,
                    uint32_t *counts, cudaStream_t st)
 {
-  kHitsAny<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, st>>>(g, attr, filter, depth, vr, numValues, values, n,
+  int dev = 0, sms = 0;
+  cudaCheck(cudaGetDevice(&dev), "cudaGetDevice");
+  cudaCheck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attribute");
+  const bool many = n > (uint64_t)sms * 2 * kBlock && numValues <= 4 && filter != kFilterCubic;
+  const auto k    = many ? kHitsAny<3> : kHitsAny<1>;
+  k<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, st>>>(g, attr, filter, depth, vr, numValues, values, n,
                                                                      origins, directions, tRanges, maxPerRay, out,
                                                                      counts);
   cudaCheck(cudaGetLastError(), "hit kernel launch");

@@ -1,6 +1,10 @@
 // Sampling of several attributes that differ in type, or at few points
 // (useTilesM, k_sample.cu) (vklComputeSampleMN, VdbSampler.ispc:131-252): one
 // point per thread through the run-time dispatch on type and filter.
+
+// Every type and filter is inlined in one kernel, whose registers the fused
+// form of the tricubic sums would decide.
+#define VKL_TRICUBIC_PLAIN 1
 #include "sample_kernels.cuh"
 
 namespace vklcuda {

@@ -111,11 +111,13 @@ __global__ void __launch_bounds__(kBlock, kDenseIntervalMinBlocks)
   if (rangesShared && threadIdx.x < vr.numRanges)
     sr[threadIdx.x] = make_float2(__ldg(vr.ranges + 2 * threadIdx.x), __ldg(vr.ranges + 2 * threadIdx.x + 1));
   __syncthreads();
-  // the first ranges in registers, absent ones as ranges nothing overlaps
+  // the first ranges in registers, absent ones as NaN, which nothing overlaps
+  // (+inf .. -inf would overlap a cell of all values)
   float2 rr[kIvRegRanges];
 #pragma unroll
   for (int i = 0; i < kIvRegRanges; ++i)
-    rr[i] = rangesShared && (uint32_t)i < vr.numRanges ? sr[i] : make_float2(kPosInf, -kPosInf);
+    rr[i] = rangesShared && (uint32_t)i < vr.numRanges ? sr[i]
+                                                       : make_float2(__builtin_nanf(""), __builtin_nanf(""));
   const int lane    = threadIdx.x & 31;
   float *const rows = rowsAll + (threadIdx.x & ~31) * kIvPitch;
   float *const row  = rows + lane * kIvPitch;

@@ -61,3 +61,22 @@ def test_time_with_many_ranges(vkl):
             best = min(best, a.elapsed_time(b))
         times.append(best)
     assert times[1] < 1.8 * times[0], times
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 33])
+def test_ranges_that_nothing_overlaps(vkl, device, oracle, count):
+    """NaN ranges overlap nothing, not even cells that hold both infinities."""
+    vox = sinusoid_field((40, 33, 26), seed=5)
+    vox[::3, ::5, ::4] = np.inf
+    vox[1::3, ::5, ::4] = -np.inf
+    ref = oracle.OracleVolume.dense_volume(vox)
+    b = ref.info()["bounds"]
+    o, d, t = random_rays(300, b[:3], b[3:], seed=3)
+    smp = vkl.Sampler(vkl.structured_regular(device, vox))
+    for vr in (np.full((count, 2), np.nan, np.float32), np.array([[np.nan, np.nan]] * (count - 1) + [[0, 0.5]], np.float32)):
+        ctx = vkl.IntervalIteratorContext(smp, value_ranges=vr)
+        want, wcnt = ref.intervals(o, d, t, value_ranges=vr, max_intervals=64)
+        got, cnt = ctx.iterate_n(o, d, t, max_per_ray=64)
+        np.testing.assert_array_equal(cnt, wcnt)
+        for r in range(len(cnt)):
+            np.testing.assert_array_equal(bits(got[r, :cnt[r]]), bits(want[r, :cnt[r]]), err_msg=f"ray {r}")

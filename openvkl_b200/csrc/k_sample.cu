@@ -9,7 +9,10 @@ namespace {
 // Which calls take one point per thread (sample_direct.cuh) and which the
 // sorted tiles.  Up to kDirectPoints everything runs faster direct (16,000
 // points: 9.7 -> 6.5 us float, 17.1 -> 6.3 us VDB, 19.7 -> 6.4 us tricubic;
-// 600,000: 36 -> 30, 26 -> 20, 67 -> 55 us).  Of larger calls:
+// 600,000: 36 -> 30, 26 -> 20, 67 -> 55 us), but tricubic floats without an
+// atlas, whose bricked loads the sort brings together: camera-ray samples up
+// to kDirectBricked (262,000 in 40 per ray 51 -> 35 us, 1M 132 -> 160; other
+// types 0.8 to 0.93 of the sort's time at 1M).  Of larger calls:
 //  - nearest: one voxel per point, nothing for a sort to gain (12M camera-ray
 //    samples 138 -> 75 us, random points 283 -> 262 us);
 //  - tricubic through an atlas (14.4M camera-ray samples 1004 -> 912 us; by
@@ -30,11 +33,13 @@ namespace {
 //    rays 242 direct; only points that all lie in active leaves are 4 % faster
 //    in tiles, 885 against 922 us);
 //  - sparse without a leaf map and sparse tricubic keep the tiles.
-constexpr uint64_t kDirectPoints = uint64_t(1) << 20;
+constexpr uint64_t kDirectPoints  = uint64_t(1) << 20;
+constexpr uint64_t kDirectBricked = uint64_t(3) << 17;
 
 bool useDirect(const DevGrid &g, int filter, uint32_t maxDepth, uint64_t n, uint32_t attr, const PointLayout &layout)
 {
-  if (n < kDirectPoints || filter == kFilterNearest)
+  const bool bricked = g.dense && filter == kFilterCubic && g.type[attr] == kFloat && !tilesUseAtlas(g, attr);
+  if (n < (bricked ? kDirectBricked : kDirectPoints) || filter == kFilterNearest)
     return true;
   // (2.4M random points of shorts 57 -> 49 us, camera rays of bytes even)
   if (g.dense && filter == kFilterLinear && g.type[attr] != kFloat && n < 4 * kDirectPoints)

@@ -204,8 +204,35 @@ void Device::ensurePipeline()
   }
 }
 
+namespace {
+// Live devices, whose pooled atlases an allocation may claim.
+std::mutex g_devicesMutex;
+std::vector<Device *> g_devices;
+}  // namespace
+
+void dropPooledAtlases()
+{
+  int current = 0;
+  if (cudaGetDevice(&current) != cudaSuccess)
+    return;
+  std::lock_guard<std::mutex> lock(g_devicesMutex);
+  for (Device *d : g_devices)
+    if (d->cudaDevice == current)
+      d->dropAtlases();
+}
+
+Device::Device()
+{
+  std::lock_guard<std::mutex> lock(g_devicesMutex);
+  g_devices.push_back(this);
+}
+
 Device::~Device()
 {
+  {
+    std::lock_guard<std::mutex> lock(g_devicesMutex);
+    g_devices.erase(std::remove(g_devices.begin(), g_devices.end(), this), g_devices.end());
+  }
   if (!copyIn)
     return;
   cudaStreamSynchronize(copyIn);
@@ -746,11 +773,13 @@ void Volume::commitDense()
   const uint32_t planesPerRow =
       device->textureSampling ? atlasPlanesPerRow(device->cudaDevice, udims[0], udims[1], udims[2]) : 0;
   grid.atlasPlanesPerRow = planesPerRow ? planesPerRow : 1;
+  // the voxels of all attributes before the first atlas, so that the atlases
+  // only take memory that the commit does not need
   for (uint32_t a = 0; a < grid.numAttributes; ++a) {
-    const size_t es  = sizeOfType(attrs[a]->type);
-    DeviceBuffer *bb = newBuffer(nb * es);
-    grid.data[a] = bb->ptr;
+    grid.data[a] = newBuffer(nb * sizeOfType(attrs[a]->type))->ptr;
     grid.type[a] = attrs[a]->type;
+  }
+  for (uint32_t a = 0; a < grid.numAttributes; ++a) {
     uint64_t surf = 0;
     if (planesPerRow && attrs[a]->type != VKL_DOUBLE) {
       const uint32_t w = planesPerRow * udims[0], h = (udims[2] + planesPerRow - 1) / planesPerRow * udims[1];
@@ -770,7 +799,7 @@ void Volume::commitDense()
     } else if (atlases[a]) {
       device->giveAtlas(std::move(atlases[a]));
     }
-    launchDenseBrickRanges(attrs[a]->dev, attrs[a]->type, bb->ptr, udims, grid.superX, grid.superY,
+    launchDenseBrickRanges(attrs[a]->dev, attrs[a]->type, (void *)grid.data[a], udims, grid.superX, grid.superY,
                            grid.background[a], leafRanges.as<float>(), surf, grid.atlasPlanesPerRow,
                            denormalFlags + a, st);
     launchPropagateRanges(grid, a, grid.numLeaves, nullptr, leafRanges.as<float>(),

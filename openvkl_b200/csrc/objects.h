@@ -122,8 +122,12 @@ struct Ref {
   explicit operator bool() const { return p != nullptr; }
 };
 
+// Frees the atlases that devices on the current GPU keep for later commits.
+void dropPooledAtlases();
+
 // ---------------------------------------------------------------------------
-// Device memory owned by an object.
+// Device memory owned by an object.  An allocation that finds no memory is
+// tried again without the pooled atlases.
 // ---------------------------------------------------------------------------
 struct DeviceBuffer {
   void *ptr    = nullptr;
@@ -143,7 +147,17 @@ struct DeviceBuffer {
   {
     release();
     if (n) {
-      cudaCheck(cudaMalloc(&ptr, n), "cudaMalloc");
+      cudaError_t e = cudaMalloc(&ptr, n);
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        dropPooledAtlases();
+        e = cudaMalloc(&ptr, n);
+      }
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        ptr = nullptr;
+      }
+      cudaCheck(e, "cudaMalloc");
       bytes = n;
     }
   }
@@ -233,6 +247,7 @@ bool launchSampleBinned(const DevGrid &g, int filter, uint64_t n, const float *p
 struct TextureAtlas;
 
 struct Device {
+  Device();
   // 1 for the application's handle plus 1 per live object of the device.
   std::atomic<int> refs{1};
   void refInc() { refs.fetch_add(1); }
@@ -284,7 +299,7 @@ struct Device {
   // Atlases of released or re-shaped volumes, kept for the next commit of
   // an atlas of the same size (a volume released and created again each
   // frame then allocates none); at most kAtlasPool are kept, and all are
-  // dropped when an atlas allocation fails.
+  // dropped when an allocation finds no memory.
   static constexpr size_t kAtlasPool = 2;
   std::mutex atlasMutex;
   std::vector<std::unique_ptr<TextureAtlas>> atlasPool;
@@ -377,6 +392,9 @@ struct Volume : ManagedObject {
   // new data of the same shape allocates nothing); the rest are freed when
   // the commit ends.
   std::vector<std::unique_ptr<DeviceBuffer>> recycled;
+  // Where there is no memory for a buffer, the previous commit's atlases,
+  // which a volume can do without, make room (a commit makes its own only
+  // once it has all its buffers).
   DeviceBuffer *newBuffer(size_t bytes)
   {
     for (auto it = recycled.begin(); it != recycled.end(); ++it)
@@ -386,7 +404,19 @@ struct Volume : ManagedObject {
         return buffers.back().get();
       }
     buffers.emplace_back(new DeviceBuffer());
-    buffers.back()->alloc(bytes);
+    try {
+      buffers.back()->alloc(bytes);
+    } catch (const VklError &e) {
+      bool any = false;
+      for (auto &a : atlases)
+        if (a) {
+          a.reset();
+          any = true;
+        }
+      if (e.code != VKL_OUT_OF_MEMORY || !any)
+        throw;
+      buffers.back()->alloc(bytes);
+    }
     return buffers.back().get();
   }
 

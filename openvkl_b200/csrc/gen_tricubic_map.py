@@ -14,7 +14,8 @@ A term w * c is an exact product when w is a power of two, so adding it is one
 fused multiply-add with the same single rounding; the other weights (3, 6, 9,
 12, 18, 27) round the product first, as the reference does: w * c is
 2^k * (odd * c), rounded once in odd * c, and the terms of a column that share
-an odd factor share that product.
+an odd factor share that product.  The two forms differ where a product w * c
+overflows: fused, the sum may still be finite.
 
 Run:  python openvkl_b200/csrc/gen_tricubic_map.py
 """
@@ -48,15 +49,14 @@ def main():
         "// GENERATED by gen_tricubic_map.py -- do not edit.",
         "// Lekien-Marsden tricubic constraint->coefficient map (see generator).",
         "#pragma once",
-        "// VKL_TRICUBIC_PLAIN: the sums as written, for translation units that inline",
-        "// the filter many times (the fused form takes the compiler far longer).",
-        "#ifdef VKL_TRICUBIC_PLAIN",
+        "// The sums as written.",
         "#define VKL_TRICUBIC_MAP(CTR, COEF) \\",
     ]
     for r, row in enumerate(tricubic_rows()):
         terms = " + ".join(f"({w:.1f}f) * CTR[{c}]" for c, w in row)
         lines.append(f"  COEF[{r}] = {terms}; \\")
-    lines += ["", "#else", "#define VKL_TRICUBIC_MAP(CTR, COEF) \\"]
+    lines += ["", "// The same sums with fused multiply-adds, for constraints whose products do",
+              "// not overflow (generator).", "#define VKL_TRICUBIC_MAP_FUSED(CTR, COEF) \\"]
     for r, row in enumerate(tricubic_rows()):
         e = ""
         for c, w in row:
@@ -73,7 +73,7 @@ def main():
             else:
                 e = f"__fmaf_rn({sign * two}.0f, {x}, {e})"
         lines.append(f"  COEF[{r}] = {e}; \\")
-    lines += ["", "#endif"]
+    lines.append("")
     out = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tricubic_map.cuh")
     with open(out, "w") as f:
         f.write("\n".join(lines) + "\n")

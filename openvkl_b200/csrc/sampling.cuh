@@ -928,6 +928,9 @@ __device__ __forceinline__ f3 gradientLinear(const Field &F, f3 p)
 // tricubic_map.cuh (generated, with a test that pins it to the reference).
 #include "tricubic_map.cuh"
 
+// PLAIN: the coefficient sums as written, else with fused multiply-adds
+// (tricubic_map.cuh).
+template <bool PLAIN>
 __device__ __forceinline__ void tricubicCoefficients(const float s[64], float coef[64])
 {
 #define S(X, Y, Z) s[((X) + 1) * 16 + ((Y) + 1) * 4 + ((Z) + 1)]
@@ -951,17 +954,20 @@ __device__ __forceinline__ void tricubicCoefficients(const float s[64], float co
                             S(x + 1, y + 1, z - 1) + S(x + 1, y + 1, z + 1));
   }
 #undef S
-  VKL_TRICUBIC_MAP(ctr, coef)
+  if constexpr (PLAIN) {
+    VKL_TRICUBIC_MAP(ctr, coef)
+  } else {
+    VKL_TRICUBIC_MAP_FUSED(ctr, coef)
+  }
 }
 
-template <class Field>
-__device__ __forceinline__ float sampleCubic(const Field &F, f3 p)
+// The tricubic polynomial of the taps s at (dx, dy, dz) of their cell, and its
+// gradient.
+template <bool PLAIN>
+__device__ __forceinline__ float cubicValue(const float s[64], float dx, float dy, float dz)
 {
-  const int32_t ix = ifloor(p.x), iy = ifloor(p.y), iz = ifloor(p.z);
-  float s[64], c[64];
-  F.stencil64(ix, iy, iz, s);
-  tricubicCoefficients(s, c);
-  const float dx = p.x - (float)ix, dy = p.y - (float)iy, dz = p.z - (float)iz;
+  float c[64];
+  tricubicCoefficients<PLAIN>(s, c);
   const float X[4] = {1.f, dx, dx * dx, dx * dx * dx};
   const float Y[4] = {1.f, dy, dy * dy, dy * dy * dy};
   const float Z[4] = {1.f, dz, dz * dz, dz * dz * dz};
@@ -976,14 +982,11 @@ __device__ __forceinline__ float sampleCubic(const Field &F, f3 p)
   return r;
 }
 
-template <class Field>
-__device__ __forceinline__ f3 gradientCubic(const Field &F, f3 p)
+template <bool PLAIN>
+__device__ __forceinline__ f3 cubicGradient(const float s[64], float dx, float dy, float dz)
 {
-  const int32_t ix = ifloor(p.x), iy = ifloor(p.y), iz = ifloor(p.z);
-  float s[64], c[64];
-  F.stencil64(ix, iy, iz, s);
-  tricubicCoefficients(s, c);
-  const float dx = p.x - (float)ix, dy = p.y - (float)iy, dz = p.z - (float)iz;
+  float c[64];
+  tricubicCoefficients<PLAIN>(s, c);
   const float X[4] = {1.f, dx, dx * dx, dx * dx * dx};
   const float Y[4] = {1.f, dy, dy * dy, dy * dy * dy};
   const float Z[4] = {1.f, dz, dz * dz, dz * dz * dz};
@@ -1003,6 +1006,70 @@ __device__ __forceinline__ f3 gradientCubic(const Field &F, f3 p)
           r.z += cc * (float)k * X[i] * Y[j] * Z[k - 1];
       }
   return r;
+}
+
+// VKL_TRICUBIC_PLAIN: for translation units that inline the filter many times
+// (the fused form takes the compiler far longer).
+#ifdef VKL_TRICUBIC_PLAIN
+constexpr bool kTricubicPlain = true;
+#else
+constexpr bool kTricubicPlain = false;
+// Taps of 2^100 and more (the weights' products stay far from overflow below
+// it, and both forms round alike there) take the sums as written, out of line.
+__device__ __forceinline__ bool tricubicLarge(const float s[64])
+{
+  float m = 0.f;
+#pragma unroll
+  for (int i = 0; i < 64; ++i)
+    m = fmaxf(m, fabsf(s[i]));
+  return m >= 0x1p100f;
+}
+static __device__ __noinline__ float cubicValueLarge(const float *s, float dx, float dy, float dz)
+{
+  return cubicValue<true>(s, dx, dy, dz);
+}
+static __device__ __noinline__ f3 cubicGradientLarge(const float *s, float dx, float dy, float dz)
+{
+  return cubicGradient<true>(s, dx, dy, dz);
+}
+#endif
+
+template <class Field>
+__device__ __forceinline__ float sampleCubic(const Field &F, f3 p)
+{
+  const int32_t ix = ifloor(p.x), iy = ifloor(p.y), iz = ifloor(p.z);
+  const float dx = p.x - (float)ix, dy = p.y - (float)iy, dz = p.z - (float)iz;
+  float s[64];
+  F.stencil64(ix, iy, iz, s);
+#ifndef VKL_TRICUBIC_PLAIN
+  if (tricubicLarge(s)) {
+    float copy[64];  // keeps s itself in registers
+#pragma unroll
+    for (int i = 0; i < 64; ++i)
+      copy[i] = s[i];
+    return cubicValueLarge(copy, dx, dy, dz);
+  }
+#endif
+  return cubicValue<kTricubicPlain>(s, dx, dy, dz);
+}
+
+template <class Field>
+__device__ __forceinline__ f3 gradientCubic(const Field &F, f3 p)
+{
+  const int32_t ix = ifloor(p.x), iy = ifloor(p.y), iz = ifloor(p.z);
+  const float dx = p.x - (float)ix, dy = p.y - (float)iy, dz = p.z - (float)iz;
+  float s[64];
+  F.stencil64(ix, iy, iz, s);
+#ifndef VKL_TRICUBIC_PLAIN
+  if (tricubicLarge(s)) {
+    float copy[64];
+#pragma unroll
+    for (int i = 0; i < 64; ++i)
+      copy[i] = s[i];
+    return cubicGradientLarge(copy, dx, dy, dz);
+  }
+#endif
+  return cubicGradient<kTricubicPlain>(s, dx, dy, dz);
 }
 
 template <class Field>

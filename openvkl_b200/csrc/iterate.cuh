@@ -170,10 +170,10 @@ __device__ __forceinline__ void ddaCell(const Dda &d, uint32_t l, int32_t &x, in
 // Runtime-level DDA: the same state and steps with the per-level arrays
 // indexed by the level at run time (local memory), each step's t and index
 // increments stored per level.  One copy of the step code serves every level:
-// the form of the per-call iterators and of the generic hit kernel, whose
-// state lives in memory or whose code is large already.  The batched kernels
-// keep their levels in registers (Dda above, DdaCell below; k_hits.cu).  All
-// compute the same values.
+// the form of the hit iterators outside k_hits.cu and of the __device__ API,
+// whose state lives in memory or whose code is large already.  The per-call
+// interval iterator and the batched kernels keep their levels in registers
+// (Dda above, DdaCell below; k_hits.cu).  All compute the same values.
 struct DdaDyn {
   uint32_t level;
   float t;
@@ -714,16 +714,13 @@ __device__ inline float bisect(const Ctx &c, float t0, float s0, float t, float 
 
 // intersectSurfacesBisection (Iterator.ih): march [tLo, tHi) with the
 // interval's nominal step, find the first iso crossing, refine it by
-// bisection.  With LOOKAHEAD > 1 the t of the next LOOKAHEAD march steps
-// are computed first (the same serial additions) and their samples issued
-// together, so their loads overlap; the steps are then examined in order
-// exactly as the one-step loop would, and samples past a hit are discarded.
+// bisection.
 //
 // (cacheT, cacheS) is the last march sample of the ray, (t, sampleAt(t)): an
 // interval that starts where the previous one's march ended (the usual case:
 // the DDA's intervals abut and the march's last step lands on the interval
 // end) reuses it instead of sampling the same t again.
-template <int LOOKAHEAD, class Ctx>
+template <class Ctx>
 __device__ inline bool intersectBisection(const Ctx &c, float tLo, float tHi, float step, uint32_t numValues,
                                           const float *values, DevHit &hit, float &cacheT, float &cacheS)
 {
@@ -733,72 +730,50 @@ __device__ inline bool intersectBisection(const Ctx &c, float tLo, float tHi, fl
     t0 += maxx(1e-5f, 1e-5f * step);
     s0 = c.sampleAt(t0);
   }
-  uint32_t march = 0;
-  while (t0 < tHi && march < kMaxMarchSteps) {
-    float tk[LOOKAHEAD], hk[LOOKAHEAD], sk[LOOKAHEAD];
-    int kn   = 0;
-    float tt = t0;
-#pragma unroll
-    for (int k = 0; k < LOOKAHEAD; ++k)
-      if (tt < tHi && march + (uint32_t)k < kMaxMarchSteps) {
-        hk[k] = minx(step, tHi - tt);
-        tk[k] = tt + hk[k];
-        tt    = tk[k];
-        kn    = k + 1;
-      }
-#pragma unroll
-    for (int k = 0; k < LOOKAHEAD; ++k)
-      if (k < kn)
-        sk[k] = c.sampleAt(tk[k]);
-    cacheT = tk[kn - 1];
-    cacheS = sk[kn - 1];
-#pragma unroll
-    for (int k = 0; k < LOOKAHEAD; ++k) {
-      if (k >= kn)
-        break;
-      const float h = hk[k];
-      const float t = tk[k];
-      float s       = sk[k];
-      float ts      = t;
-      for (int it = 0; (float)it < 10.f && isnan(s) && ts > t0; ++it) {
-        ts -= maxx(1e-5f, 1e-5f * step);
-        s = c.sampleAt(ts);
-      }
-      float tHit = kPosInf, eps = kPosInf, value = kPosInf;
-      for (uint32_t i = 0; i < numValues; ++i) {
-        const float vi = __ldg(values + i);
-        if (fabsf(s0 - vi) < 1e-6f) {
-          if (t0 < tHit && t0 <= tHi) {
-            tHit  = t0;
-            value = vi;
-            eps   = 0.125f * step;
-          }
-        } else if (!isnan(s0 + s) && (vi - s0) * (vi - s) < 0.f) {
-          const float tIso = bisect(c, t0, s0, ts, s, vi, minx(1e-6f, 0.01f * h));
-          if (tIso < tHit && tIso <= tHi) {
-            tHit  = tIso;
-            value = vi;
-            eps   = 0.125f * step;
-          }
-        }
-        if (t == tHi && fabsf(s - vi) < 1e-6f) {
-          if (ts < tHit && ts <= tHi) {
-            tHit  = ts;
-            value = vi;
-            eps   = 0.125f * step;
-          }
-        }
-      }
-      if (tHit < kPosInf) {
-        hit.t       = tHit;
-        hit.sample  = value;
-        hit.epsilon = eps * sqrtf(c.d.x * c.d.x + c.d.y * c.d.y + c.d.z * c.d.z);
-        return true;
-      }
-      t0 = t;
-      s0 = s;
+  for (uint32_t march = 0; t0 < tHi && march < kMaxMarchSteps; ++march) {
+    const float h = minx(step, tHi - t0);
+    const float t = t0 + h;
+    float s       = c.sampleAt(t);
+    cacheT        = t;
+    cacheS        = s;
+    float ts      = t;
+    for (int it = 0; (float)it < 10.f && isnan(s) && ts > t0; ++it) {
+      ts -= maxx(1e-5f, 1e-5f * step);
+      s = c.sampleAt(ts);
     }
-    march += (uint32_t)kn;
+    float tHit = kPosInf, eps = kPosInf, value = kPosInf;
+    for (uint32_t i = 0; i < numValues; ++i) {
+      const float vi = __ldg(values + i);
+      if (fabsf(s0 - vi) < 1e-6f) {
+        if (t0 < tHit && t0 <= tHi) {
+          tHit  = t0;
+          value = vi;
+          eps   = 0.125f * step;
+        }
+      } else if (!isnan(s0 + s) && (vi - s0) * (vi - s) < 0.f) {
+        const float tIso = bisect(c, t0, s0, ts, s, vi, minx(1e-6f, 0.01f * h));
+        if (tIso < tHit && tIso <= tHi) {
+          tHit  = tIso;
+          value = vi;
+          eps   = 0.125f * step;
+        }
+      }
+      if (t == tHi && fabsf(s - vi) < 1e-6f) {
+        if (ts < tHit && ts <= tHi) {
+          tHit  = ts;
+          value = vi;
+          eps   = 0.125f * step;
+        }
+      }
+    }
+    if (tHit < kPosInf) {
+      hit.t       = tHit;
+      hit.sample  = value;
+      hit.epsilon = eps * sqrtf(c.d.x * c.d.x + c.d.y * c.d.y + c.d.z * c.d.z);
+      return true;
+    }
+    t0 = t;
+    s0 = s;
   }
   return false;
 }
@@ -825,7 +800,7 @@ __device__ inline void hitInit(const DevGrid &g, uint32_t depth, f3 o, f3 d, flo
 }
 
 // One vklIterateHit call (DefaultIterator.ispc:168-258).
-template <int LOOKAHEAD, class Hook>
+template <class Hook>
 __device__ inline bool hitNextWith(const DevGrid &g, const Hook &hook, uint32_t attr, const DevValueRanges &vr,
                                    uint32_t numValues, const float *values, HitIt &h, DevHit &hit)
 {
@@ -849,8 +824,7 @@ __device__ inline bool hitNextWith(const DevGrid &g, const Hook &hook, uint32_t 
       return false;
     }
     hit.t = kPosInf;
-    if (intersectBisection<LOOKAHEAD>(c, h.cur.t0, h.cur.t1, h.cur.nominalDeltaT, numValues, values, hit,
-                                      h.cacheT, h.cacheS)) {
+    if (intersectBisection(c, h.cur.t0, h.cur.t1, h.cur.nominalDeltaT, numValues, values, hit, h.cacheT, h.cacheS)) {
       h.cur.t0         = hit.t + hit.epsilon;
       h.lastHitOffsetT = hit.t + hit.epsilon;
       return true;
@@ -863,8 +837,7 @@ __device__ inline bool hitNext(const DevGrid &g, int filter, uint32_t attr, uint
                                const DevValueRanges &vr, uint32_t numValues, const float *values,
                                HitIt &h, DevHit &hit, float time = 0.f)
 {
-  return hitNextWith<1>(g, AnySampleHook{&g, filter, attr, sampleDepth, time}, attr, vr, numValues, values, h,
-                        hit);
+  return hitNextWith(g, AnySampleHook{&g, filter, attr, sampleDepth, time}, attr, vr, numValues, values, h, hit);
 }
 
 }  // namespace vklcuda

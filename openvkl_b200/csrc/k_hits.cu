@@ -34,8 +34,9 @@ namespace {
 
 constexpr int kBlock     = 128;
 constexpr int kHitValues = 32;  // isovalues kept in shared memory
-// 4 x 128 threads per SM: 128 registers without spills (400,003 random rays,
-// 1024^3 shells: 8.75 ms; three: 10.3; five, spilling: 15.1 ms before the
+// 4 x 128 threads per SM: 128 registers, without spills for float leaves and
+// with 24 to 72 bytes of them for coded ones (400,003 random rays, 1024^3
+// shells, float: 8.75 ms; three: 10.3; five, spilling: 15.1 ms before the
 // warp's ray pool).
 constexpr int kHitMinBlocks = 4;
 

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kBlock, CTAS) kHitsAny(const __grid_constant__
   uint32_t c = 0;
   DevHit hit;
   const AnySampleHook hook{&g, filter, attr, kNumLevels - 1};
-  while (c < kMaxHitsPerRay && hitNextWith<1>(g, hook, attr, vr, numValues, values, h, hit)) {
+  while (c < kMaxHitsPerRay && hitNextWith(g, hook, attr, vr, numValues, values, h, hit)) {
     if (c < maxPerRay)
       out[r * maxPerRay + c] = hit;
     ++c;

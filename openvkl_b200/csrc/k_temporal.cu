@@ -22,7 +22,21 @@ namespace {
 constexpr int kTemporalBlock = kDirectBlock;
 constexpr float kInfF     = __builtin_huge_valf();
 
-// LAYOUT: whether the points come by rays is read from `layout` (directPoint): a
+// The point of a thread by rays of S samples (at least 8): as directPoint's, but
+// groups of 8 rays follow one another without gaps, so that the grid hardly
+// depends on S, which the host does not know.
+__device__ __forceinline__ uint64_t rayPoint(uint32_t S)
+{
+  const uint32_t u = blockIdx.x * (kTemporalBlock / 8);  // samples of 8 rays before the block
+  uint32_t group = u / S, e = (u - group * S) * 8 + threadIdx.x;
+  while (e >= 8 * S) {
+    e -= 8 * S;
+    ++group;
+  }
+  return ((uint64_t)group * 8 + (e & 7u)) * S + (e >> 3);
+}
+
+// LAYOUT: whether the points come by rays is read from `layout` (rayPoint): a
 // warp's 32 points x 16 time samples are then close together (14.8M camera-ray
 // samples, 64 per ray, of 256x250x200 floats x 4 steps: 437 -> 335 us, 14M at
 // 200 per ray 377 -> 303).  Rays of fewer samples have them too far apart to
@@ -54,8 +68,8 @@ __global__ void __launch_bounds__(kTemporalBlock)
                     float *__restrict__ out)
 {
   const uint32_t S = LAYOUT && layout->order >= kTemporalRays ? layout->order : 0u;
-  uint64_t i;
-  if (directPoint(blockIdx.x, S, n, i))
+  const uint64_t i = S ? rayPoint(S) : (uint64_t)blockIdx.x * kTemporalBlock + threadIdx.x;
+  if (i < n)
     sampleTemporal<T, FILTER, GRAD>(g, i, pts, times, attr, out);
 }
 

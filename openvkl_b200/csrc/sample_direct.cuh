@@ -13,31 +13,27 @@ namespace vklcuda {
 
 constexpr int kDirectBlock = 128;
 
-// The point of a thread: point by point, or by rays (S samples each, at least
-// 8): 8 neighbouring rays sample by sample, so a warp takes 4 consecutive
-// samples of each, which lie closer together than 32 samples of one ray.
-// Groups of 8 rays follow one another without gaps.
-__device__ __forceinline__ bool directPoint(uint32_t block, uint32_t S, uint64_t n, uint64_t &i)
+// The point of a thread: point by point, or by rays (S samples each): a block
+// takes 16 consecutive samples of 8 neighbouring rays and a warp 4 of each,
+// which lie closer together than 32 samples of one ray.
+__device__ __forceinline__ bool directPoint(uint32_t S, uint64_t n, uint64_t &i)
 {
   if (!S) {
-    i = (uint64_t)block * kDirectBlock + threadIdx.x;
+    i = (uint64_t)blockIdx.x * kDirectBlock + threadIdx.x;
     return i < n;
   }
-  const uint32_t u = block * (kDirectBlock / 8);  // samples of 8 rays before the block
-  uint32_t group = u / S, e = (u - group * S) * 8 + threadIdx.x;
-  while (e >= 8 * S) {
-    e -= 8 * S;
-    ++group;
-  }
-  i = ((uint64_t)group * 8 + (e & 7u)) * S + (e >> 3);
-  return i < n;
+  constexpr uint32_t kSamples = kDirectBlock / 8;
+  const uint32_t segs = (S + kSamples - 1) / kSamples, rays = blockIdx.x / segs;
+  const uint32_t s = (blockIdx.x - rays * segs) * kSamples + (threadIdx.x >> 3);
+  i                = ((uint64_t)rays * 8 + (threadIdx.x & 7u)) * S + s;
+  return s < S && i < n;
 }
 inline unsigned directBlocks(uint32_t S, uint64_t n)
 {
   if (!S)
     return (unsigned)((n + kDirectBlock - 1) / kDirectBlock);
   constexpr uint32_t kSamples = kDirectBlock / 8;
-  return (unsigned)((((n + S - 1) / S + 7) / 8 * S + kSamples - 1) / kSamples);
+  return (unsigned)(((n + S - 1) / S + 7) / 8 * ((S + kSamples - 1) / kSamples));
 }
 
 // CTAs of 128 threads per SM: 10 (48 registers) is between the best of camera
@@ -55,9 +51,13 @@ struct DirectTraits<MappedField<T>, kFilterLinear> {
 };
 
 template <class Field, int FILTER, bool GRAD>
-__device__ __forceinline__ void sampleDirect(const DevGrid &g, uint32_t maxDepth, uint64_t i,
-                                             const float *__restrict__ pts, uint32_t attr, float *__restrict__ out)
+__global__ void __launch_bounds__(kDirectBlock, DirectTraits<Field, FILTER>::kMinBlocks)
+    kSampleDirect(const __grid_constant__ DevGrid g, uint32_t maxDepth, uint32_t S, uint64_t n,
+                  const float *__restrict__ pts, uint32_t attr, float *__restrict__ out)
 {
+  uint64_t i;
+  if (!directPoint(S, n, i))
+    return;
   const float *x = pts + 3 * i;
   const f3 p     = xfmPoint(g.objectToIndex, f3{__ldcs(x), __ldcs(x + 1), __ldcs(x + 2)});
   const Field F  = makeField<Field>(g, attr, maxDepth);
@@ -74,16 +74,6 @@ __device__ __forceinline__ void sampleDirect(const DevGrid &g, uint32_t maxDepth
   } else {
     __stcs(out + i, filterAt<Field, FILTER>(F, g.constantCellData != 0, p));
   }
-}
-
-template <class Field, int FILTER, bool GRAD>
-__global__ void __launch_bounds__(kDirectBlock, DirectTraits<Field, FILTER>::kMinBlocks)
-    kSampleDirect(const __grid_constant__ DevGrid g, uint32_t maxDepth, uint32_t S, uint64_t n,
-                  const float *__restrict__ pts, uint32_t attr, float *__restrict__ out)
-{
-  uint64_t i;
-  if (directPoint(blockIdx.x, S, n, i))
-    sampleDirect<Field, FILTER, GRAD>(g, maxDepth, i, pts, attr, out);
 }
 
 struct DirectLaunch {

@@ -20,7 +20,7 @@
 // completes a ray takes the next one its warp has left, so neither a lane
 // nor a warp idles behind the longest ray (12.0 -> 9.3 ms).
 // 400,003 random rays through the 1024^3 shells, two isovalues: 27.3 -> 8.75
-// ms.  Bound by instruction issue of diverging lanes (9 of 32 active).
+// ms.  Bound by instruction issue of diverging lanes (6 of 32 active).
 #include <algorithm>
 #include <type_traits>
 

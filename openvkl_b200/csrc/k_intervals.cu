@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kBlock, kIntervalMinBlocks) kIntervals(const _
 // memory (odd pitch: the lanes' rows start in distinct banks) and the warp
 // writes the rows out together, 8 lanes per ray on sector-aligned words:
 // 1280x721 camera rays through 512x500x512 voxels, two value ranges, 96 slots
-// per ray: 2.74 -> 0.94 ms.  Bound by instruction issue (2.4 per cycle of
+// per ray: 2.74 -> 0.94 ms.  Bound by instruction issue (2.3 per cycle of
 // the SM).
 constexpr int kIntervalLookahead = 8;
 // 2 on the upper levels, whose cells (4096^3 and 128^3 voxels) a ray
